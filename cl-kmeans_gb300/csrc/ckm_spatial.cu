@@ -155,16 +155,21 @@ __global__ void __launch_bounds__(256) bbox_sample_kernel(const float* __restric
     for (uint32_t f = 0; f < d; ++f) {
         float lo = INFINITY, hi = -INFINITY;
         const uint32_t total = gridDim.x * 256u;
-        for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < samples; i += 4u * total) {
+        uint32_t i = blockIdx.x * 256u + threadIdx.x;
+        for (; i + 3u * total < samples; i += 4u * total) {
             float v[4];  // four samples of a thread in flight
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j)
-                v[j] = i + j * total < samples ? __ldg(P + (size_t)f * n + (uint64_t)(i + j * total) * stride) : NAN;
+            for (uint32_t j = 0; j < 4; ++j) v[j] = __ldg(P + (size_t)f * n + (uint64_t)(i + j * total) * stride);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) {
                 lo = fminf(lo, v[j]);  // NaN ignored
                 hi = fmaxf(hi, v[j]);
             }
+        }
+        for (; i < samples; i += total) {
+            const float v = __ldg(P + (size_t)f * n + (uint64_t)i * stride);
+            lo = fminf(lo, v);
+            hi = fmaxf(hi, v);
         }
         const uint32_t ol = __reduce_min_sync(0xffffffffu, ord_of(lo));
         const uint32_t oh = __reduce_max_sync(0xffffffffu, ord_of(hi));
@@ -384,30 +389,34 @@ __global__ void __launch_bounds__(RADIX) scan_partial_kernel(const uint32_t* __r
 
 // One CTA: partial[blk][digit] becomes the exclusive prefix of the digit
 // over the blocks, and row nblk the start of each digit's output range (the
-// totals of the smaller digits).  Four groups of threads take a quarter of the
-// blocks each: its sum first, then its prefixes.
+// totals of the smaller digits).  GROUPS groups of threads take a part of the
+// blocks each: its sum first, then its prefixes.  One group (of 256 threads)
+// where a single batch holds all blocks, which it then reads once.
 constexpr uint32_t TOP_GROUPS = 4;
-__global__ void __launch_bounds__(RADIX * TOP_GROUPS) scan_top_kernel(uint32_t* __restrict__ partial, uint32_t nblk) {
-    __shared__ uint32_t s_sum[TOP_GROUPS][RADIX];
+template <uint32_t GROUPS>
+__global__ void __launch_bounds__(RADIX * GROUPS) scan_top_kernel(uint32_t* __restrict__ partial, uint32_t nblk) {
+    __shared__ uint32_t s_sum[GROUPS][RADIX];
     __shared__ uint32_t s_w[RADIX / 32];
     const uint32_t t = threadIdx.x % RADIX, g = threadIdx.x / RADIX, lane = t & 31u, warp = t >> 5;
-    const uint32_t per = (nblk + TOP_GROUPS - 1) / TOP_GROUPS;
+    const uint32_t per = (nblk + GROUPS - 1) / GROUPS;
     const uint32_t g0 = min(nblk, g * per), g1 = min(nblk, g0 + per);
-    uint32_t sum = 0;
-    for (uint32_t b0 = g0; b0 < g1; b0 += SCAN_BATCH) {
-        uint32_t v[SCAN_BATCH];
-#pragma unroll
-        for (uint32_t i = 0; i < SCAN_BATCH; ++i) v[i] = b0 + i < g1 ? partial[(uint64_t)(b0 + i) * RADIX + t] : 0u;
-#pragma unroll
-        for (uint32_t i = 0; i < SCAN_BATCH; ++i) sum += v[i];
-    }
-    s_sum[g][t] = sum;
-    __syncthreads();
     uint32_t run = 0, all = 0;
+    if constexpr (GROUPS > 1) {
+        uint32_t sum = 0;
+        for (uint32_t b0 = g0; b0 < g1; b0 += SCAN_BATCH) {
+            uint32_t v[SCAN_BATCH];
 #pragma unroll
-    for (uint32_t h = 0; h < TOP_GROUPS; ++h) {
-        if (h < g) run += s_sum[h][t];
-        all += s_sum[h][t];
+            for (uint32_t i = 0; i < SCAN_BATCH; ++i) v[i] = b0 + i < g1 ? partial[(uint64_t)(b0 + i) * RADIX + t] : 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < SCAN_BATCH; ++i) sum += v[i];
+        }
+        s_sum[g][t] = sum;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t h = 0; h < GROUPS; ++h) {
+            if (h < g) run += s_sum[h][t];
+            all += s_sum[h][t];
+        }
     }
     for (uint32_t b0 = g0; b0 < g1; b0 += SCAN_BATCH) {
         uint32_t v[SCAN_BATCH];
@@ -420,6 +429,7 @@ __global__ void __launch_bounds__(RADIX * TOP_GROUPS) scan_top_kernel(uint32_t* 
                 run += v[i];
             }
     }
+    if constexpr (GROUPS == 1) all = run;
     uint32_t incl = all;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -563,20 +573,10 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
     }
 }
 
-__global__ void __launch_bounds__(256) unpermute_kernel(uint64_t n, int vec, const uint32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) unpermute_kernel(uint64_t n, const uint32_t* __restrict__ perm,
                                                         const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
-    const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x, stride = (uint64_t)gridDim.x * 256;
-    // perm and in are read once: streaming loads leave L2 to the scattered words
-    const uint64_t quads = vec ? n / 4 : 0;
-    for (uint64_t q = t; q < quads; q += stride) {
-        const uint4 p = __ldcs(reinterpret_cast<const uint4*>(perm) + q);
-        const uint4 v = __ldcs(reinterpret_cast<const uint4*>(in) + q);
-        out[p.x] = v.x;
-        out[p.y] = v.y;
-        out[p.z] = v.z;
-        out[p.w] = v.w;
-    }
-    for (uint64_t q = quads * 4 + t; q < n; q += stride) out[__ldcs(perm + q)] = __ldcs(in + q);
+    for (uint64_t q = (uint64_t)blockIdx.x * 256 + threadIdx.x; q < n; q += (uint64_t)gridDim.x * 256)
+        out[perm[q]] = in[q];
 }
 
 uint32_t grid_of(uint64_t n) {
@@ -590,7 +590,8 @@ int scan_offsets(uint32_t* counts, uint32_t* partial, uint64_t chunks, cudaStrea
     const uint32_t per = scan_rows_of(chunks);
     const uint32_t nblk = (uint32_t)((chunks + per - 1) / per);
     scan_partial_kernel<<<nblk, RADIX, 0, s>>>(counts, chunks, per, partial);
-    scan_top_kernel<<<1, RADIX * TOP_GROUPS, 0, s>>>(partial, nblk);
+    if (nblk <= SCAN_BATCH) scan_top_kernel<1><<<1, RADIX, 0, s>>>(partial, nblk);
+    else scan_top_kernel<TOP_GROUPS><<<1, RADIX * TOP_GROUPS, 0, s>>>(partial, nblk);
     scan_apply_kernel<<<nblk, RADIX, 0, s>>>(counts, chunks, per, partial, nblk);
     return 3;
 }
@@ -667,8 +668,7 @@ int launch_spatial_sort(uint32_t d, uint64_t n, const float* points, float* sort
 
 int launch_unpermute_u32(uint64_t n, const uint32_t* perm, const uint32_t* in, uint32_t* out, cudaStream_t s) {
     if (n == 0) return CKM_OK;
-    const int vec = ((reinterpret_cast<uintptr_t>(perm) | reinterpret_cast<uintptr_t>(in)) & 15u) == 0;
-    unpermute_kernel<<<grid_of(n), 256, 0, s>>>(n, vec, perm, in, out);
+    unpermute_kernel<<<grid_of(n), 256, 0, s>>>(n, perm, in, out);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CKM_OK : cuda_fail(e, "unpermute launch");
