@@ -14,6 +14,7 @@
 #include "configuration.hpp"
 #include "device.hpp"
 #include "measurement.hpp"
+#include "spatial_line.hpp"
 
 namespace Clustering {
 
@@ -108,28 +109,17 @@ private:
 
 // Whether a run uses the spatially ordered copy of its points (FP32,
 // column-major, d <= 8, k <= 32, n < 2^32).  mode: 0 = auto (additionally
-// n >= 2^20, >= 8 iterations, iterations * k >= pays_from (a third more below 2^21
-// points) and enough free device memory), 1 = whenever the shape allows, -1 =
-// never.
-//
-// pays_from: the sort costs about what three to five plain iterations do, and
-// box pruning takes off an iteration what the distances to most of the k
-// clusters take.  Loop over blobs, us, plain / sorted: single-stage n = 2^20 d =
-// 4 k = 10, 8 iterations 138 / 216, 30 500 / 532; n = 2^23 30 1623 / 1464; d = 8 k =
-// 30 8 1631 / 1469; d = 4 k = 32 15 1814 / 1237; d = 8 k = 8 15 1152 / 1494.  The
-// three-stage iterations save more (the sums of sorted points too): n = 2^20 d = 4
-// k = 10 15 629 / 536; n = 2^23 d = 4 k = 10 15 1568 / 1659, d = 8 k = 30 8 2056 / 1892.
-constexpr uint64_t SINGLE_STAGE_SPATIAL_FROM = 300, THREE_STAGE_SPATIAL_FROM = 150;
+// n >= 2^20, >= 8 iterations, `pays` (spatial_line.hpp) and enough free device
+// memory), 1 = whenever the shape allows, -1 = never.
 template <typename PointT, typename LabelT, typename MassT, bool ColMajor>
-bool spatial_order_eligible(int mode, size_t d, size_t n, size_t k, uint32_t iterations, uint64_t pays_from) {
+bool spatial_order_eligible(int mode, size_t d, size_t n, size_t k, uint32_t iterations, bool pays) {
     if (mode < 0) return false;
     if (!(std::is_same<PointT, float>::value && std::is_same<LabelT, uint32_t>::value &&
           std::is_same<MassT, uint32_t>::value && ColMajor))
         return false;
     if (d < 1 || d > 8 || k > 32 || n == 0 || n > 0xffffffffull) return false;
     if (mode > 0) return true;
-    if (n < (1ull << 20) || iterations < 8) return false;
-    if ((uint64_t)iterations * k < (n < (1ull << 21) ? pays_from * 4 / 3 : pays_from)) return false;
+    if (n < (1ull << 20) || iterations < 8 || !pays) return false;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
     const size_t need = n * d * sizeof(PointT) + n * 2 * sizeof(LabelT) + ckm_spatial_sort_workspace_bytes(n, (uint32_t)d);

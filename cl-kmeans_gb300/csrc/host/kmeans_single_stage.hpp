@@ -168,7 +168,7 @@ private:
 
     bool use_spatial_order(size_t d, size_t n, size_t k) const {
         return spatial_order_eligible<PointT, LabelT, MassT, ColMajor>(spatial_mode_, d, n, k, this->max_iterations,
-                                                                       SINGLE_STAGE_SPATIAL_FROM);
+                                                                       single_stage_spatial_pays(n, (uint32_t)k, this->max_iterations));
     }
 
     FusedLloyd<PointT, LabelT, MassT> engine_;

@@ -64,7 +64,7 @@ public:
         // the last iteration of a full run uses the caller's order
         const bool spatial =
             spatial_order_eligible<PointT, LabelT, MassT, ColMajor>(spatial_mode_, d, n, k, this->max_iterations,
-                                                                    THREE_STAGE_SPATIAL_FROM);
+                                                                    three_stage_spatial_pays(n, (uint32_t)k, this->max_iterations));
         if (spatial) {
             auto& dp = this->measurement->add_datapoint().set_name("SpatialSort");
             Event& ev = dp.add_event(q_labeling);
