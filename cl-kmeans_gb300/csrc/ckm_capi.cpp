@@ -6,6 +6,7 @@
 // launches it on the caller's stream.  No entry point allocates memory.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -92,7 +93,11 @@ int dispatch_fused_f32(const FusedF32& a, cudaStream_t s) {
         const bool lowd = lowd_sums_pay(a.n, a.d, a.k);  // (counts the labels itself)
         const int st = launch_wide_f32(a, !lowd, s);
         if (st) return st;
-        return lowd ? launch_fused_f32(a, Pass::SumsOnly, s) : launch_sums_f32(a, false, s);
+        if (lowd) return launch_fused_f32(a, Pass::SumsOnly, s);
+        // (the rows kernel adds in FP32 for every k, in one table per SM for many clusters)
+        const bool rows = rows_supported(a.d, a.k);
+        return launch_sums_f32(a, false, rows ? std::min<uint64_t>((a.n + 511) / 512, device_info().sm_count)
+                                              : sums_partials_f32(a.n, a.d, a.k), s);
     }
     if (lowd_supported(a.d, a.k)) return launch_fused_f32(a, Pass::Fused, s);
     return launch_generic_f32(a, Pass::Fused, s);
@@ -345,7 +350,7 @@ int ckm_centroid_update_f32(uint32_t d, uint64_t n, uint32_t k, const float* poi
                scratch_view(scratch, scratch_layout(d, k)), n, d, k, mode};
     cudaStream_t s = (cudaStream_t)stream;
     // (DEFER: ckm_finalize divides by the counts kept with the sums)
-    if (sums_pays_f32(n, d, k)) return launch_sums_f32(a, mode == CKM_MODE_DEFER, s);
+    if (sums_pays_f32(n, d, k)) return launch_sums_f32(a, mode == CKM_MODE_DEFER, sums_partials_f32(n, d, k), s);
     if (lowd_supported(d, k)) return launch_fused_f32(a, Pass::SumsOnly, s);
     return launch_generic_f32(a, Pass::SumsOnly, s);
 }

@@ -105,11 +105,14 @@ bool lowd_sums_pay(uint64_t n, uint32_t d, uint32_t k);  // rather than ckm_sums
 bool rows_supported(uint32_t d, uint32_t k);  // the fixed-d kernel of ckm_generic.cu
 // Per-label feature sums (ckm_sums.cu), finalised like the other passes
 // (FINALIZE divides by the counts that are in the scratch's masses); count:
-// also add the labels' counts there.
+// also add the labels' counts there.  FP32 sums start from at least `partials`
+// FP32 partial sums per entry, or are kept as pairs of floats (0: always), which
+// add up as exactly as FP64.
 // sums_pays: where a centroid update takes it.
 bool sums_pays_f32(uint64_t n, uint32_t d, uint32_t k);
 bool sums_pays_f64(uint64_t n, uint32_t d, uint32_t k);
-int launch_sums_f32(const FusedF32& a, bool count, cudaStream_t s);
+uint64_t sums_partials_f32(uint64_t n, uint32_t d, uint32_t k);
+int launch_sums_f32(const FusedF32& a, bool count, uint64_t partials, cudaStream_t s);
 int launch_sums_f64(const FusedF64& a, bool count, cudaStream_t s);
 // Labels on the tensor cores (ckm_wide.cu); count: also add the labels'
 // counts to the scratch's masses.  wide_pays: where a labeling (fused: a
