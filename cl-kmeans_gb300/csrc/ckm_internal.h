@@ -19,7 +19,7 @@ int cuda_fail(cudaError_t err, const char* where);
 // Scratch layout (all offsets 256-byte aligned):
 //   sums     double[k * d]   column-major like the centroids (f * k + c)
 //   masses   uint64[k]
-//   control  uint32[64]      [0] CTA arrival ticket, [1] error flag, [2 + g]
+//   control  uint32[64]      [0] CTA arrival ticket, [2 + g]
 //            arrival tickets of the feature groups (ckm_sums.cu)
 //   reserved SCRATCH_RESERVED bytes for d = 32 / 64, 16 <= k <= 256 (unused;
 //            the sizes callers allocate stay as they were)

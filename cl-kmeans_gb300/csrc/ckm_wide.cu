@@ -16,6 +16,10 @@
 //     the certificate, the label.
 // Each hand-over is an mbarrier, so the producers' loads, the MMAs and the
 // epilogue of neighbouring tiles overlap.
+// Every wait has a limit (2 s).  A role whose wait runs out stops the others, and
+// the CTA labels its remaining points by the reference's arithmetic with all its
+// warps: a failed hand-over costs time, not labels, so there is no error to
+// report.
 //
 // Measured (labels, before: the generic kernel, n k d chained FP32 or FP64
 // steps): n = 131072, d = 128, k = 64 330 -> 27 us; n = 300007, d = 21, k = 50
@@ -58,6 +62,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <mutex>
 
 #include "ckm_device.cuh"
@@ -77,6 +82,7 @@ constexpr uint32_t W_TILE_BYTES = WM * 128u;  // one operand tile: 128 rows of 6
 constexpr uint32_t W_NX_SLOTS = 8, W_NX_ROWS = 48;
 constexpr float W_MAX_ABS = 32768.0f;         // |x| and |c| below: no fp16 overflow
 constexpr unsigned long long W_WAIT_NS = 2000000000ull;
+constexpr uint32_t W_POLL_NS = 2000;          // a poll of a barrier suspends its thread up to this long
 
 template <typename T, typename L>
 struct WideArgs {
@@ -84,7 +90,7 @@ struct WideArgs {
     const T* centroids;
     L* labels;
     unsigned long long* msum;  // counts are added here (nullptr: not counted)
-    unsigned int* error;       // set when a bounded wait ran out (nullptr: not reported)
+    unsigned long long wait_ns;  // limit of every wait
     uint64_t n;
     uint32_t d, k, dk, kp, kblocks, stages, stages_log2, teams, tiles;
 };
@@ -95,27 +101,29 @@ __device__ __forceinline__ unsigned long long w_now_ns() {
     return t;
 }
 
-__device__ __forceinline__ bool w_try_wait(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool w_try_wait(uint32_t bar, uint32_t parity, uint32_t poll) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(20000u)
+        : "r"(bar), "r"(parity), "r"(poll)
         : "memory");
     return ok != 0;
 }
 
-// mbarrier wait with a time limit and a shared abort flag; false when another
-// role gave up or the phase did not complete in time.
-__device__ __forceinline__ bool w_wait(uint32_t bar, uint32_t parity, volatile unsigned int* abort_flag) {
-    if (w_try_wait(bar, parity)) return true;
+// mbarrier wait with a time limit and a shared flag; false when another role
+// gave the tensor cores up or the phase did not complete in time.
+__device__ __forceinline__ bool w_wait(uint32_t bar, uint32_t parity, volatile unsigned int* abort_flag,
+                                       unsigned long long limit) {
+    const uint32_t poll = limit < W_POLL_NS ? (uint32_t)limit : W_POLL_NS;
+    if (w_try_wait(bar, parity, poll)) return true;
     const unsigned long long t0 = w_now_ns();
     for (;;) {
-        if (w_try_wait(bar, parity)) return true;
+        if (w_try_wait(bar, parity, poll)) return true;
         if (*abort_flag) return false;
-        if (w_now_ns() - t0 > W_WAIT_NS) {
+        if (w_now_ns() - t0 >= limit) {
             *abort_flag = 1u;
             return false;
         }
@@ -264,6 +272,74 @@ __device__ __forceinline__ T w_distance(const T* __restrict__ P, uint64_t n, uin
     return acc;
 }
 
+// acc[j] = fma(t, t, acc[j]), t = x - row[j], for eight clusters; WORDS: row is
+// 16-byte aligned and readable to the eighth (else the first `left` are read).
+template <bool WORDS>
+__device__ __forceinline__ void w_step8(float x, const float* row, uint32_t left, float (&acc)[8]) {
+    float c[8];
+    if constexpr (WORDS) {
+        const float4 u = *reinterpret_cast<const float4*>(row), v = *reinterpret_cast<const float4*>(row + 4);
+        c[0] = u.x, c[1] = u.y, c[2] = u.z, c[3] = u.w, c[4] = v.x, c[5] = v.y, c[6] = v.z, c[7] = v.w;
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) c[j] = j < left ? __ldg(row + j) : 0.0f;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j += 2) {
+        const float2 t = sub2(make_float2(x, x), make_float2(c[j], c[j + 1]));
+        const float2 s = fma2(t, t, make_float2(acc[j], acc[j + 1]));
+        acc[j] = s.x;
+        acc[j + 1] = s.y;
+    }
+}
+template <bool WORDS>
+__device__ __forceinline__ void w_step8(double x, const double* row, uint32_t left, double (&acc)[8]) {
+    double c[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j += 2) {
+        if constexpr (WORDS) {
+            const double2 u = *reinterpret_cast<const double2*>(row + j);
+            c[j] = u.x, c[j + 1] = u.y;
+        } else {
+            c[j] = j < left ? __ldg(row + j) : 0.0;
+            c[j + 1] = j + 1 < left ? __ldg(row + j + 1) : 0.0;
+        }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        const double t = x - c[j];
+        acc[j] = fma(t, t, acc[j]);
+    }
+}
+
+// The reference's label of point p + lane by all clusters, eight at a time; the
+// centroid of feature f and cluster c is at C[f * stride + c].  Past the last
+// point the last one is labelled.
+template <typename T, bool WORDS>
+__device__ __noinline__ uint32_t w_exact32(const T* __restrict__ P, uint64_t n, uint64_t p, const T* C, uint32_t stride,
+                                           uint32_t k, uint32_t d) {
+    const uint64_t at = p + (threadIdx.x & 31u);
+    const T* first = P + (at < n ? at : n - 1);
+    T best = TypeMax<T>::v();
+    uint32_t label = 0;
+    for (uint32_t c0 = 0; c0 < k; c0 += 8) {
+        T acc[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) acc[j] = T(0);
+        const T* src = first;
+        const T* row = C + c0;
+#pragma unroll 4
+        for (uint32_t f = 0; f < d; ++f, src += n, row += stride) w_step8<WORDS>(__ldg(src), row, k - c0, acc);
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j)
+            if (c0 + j < k && acc[j] < best) {
+                best = acc[j];
+                label = c0 + j;
+            }
+    }
+    return label;
+}
+
 // EG epilogue groups, ACCS accumulators (a multiple of EG).
 template <typename T, typename L, int EG, int ACCS>
 __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const WideArgs<T, L> a) {
@@ -277,6 +353,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
     __shared__ uint32_t s_invalid[W_MAX_K / 32];
     __shared__ float s_nx[W_NX_ROWS][WM];  // partial |x|^2: [slot][part][point]
     __shared__ unsigned int s_mass[W_MAX_K];
+    __shared__ uint32_t s_next[W_EPI_WARPS];  // the first tile that an epilogue warp has not labelled
     volatile unsigned int* abort_flag = &s_abort;
 
     // the warp index as a value the compiler knows to be the same in the whole
@@ -461,7 +538,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
                 }
                 // the stage is free once the MMAs of the tile `stages` before are done
                 const uint32_t stage = it & (a.stages - 1u);
-                const bool ok = w_wait(umma::smem_u32(&bar_ae[stage]), ((it >> a.stages_log2) & 1u) ^ 1u, abort_flag);
+                const bool ok = w_wait(umma::smem_u32(&bar_ae[stage]), ((it >> a.stages_log2) & 1u) ^ 1u, abort_flag, a.wait_ns);
                 if (!__all_sync(0xffffffffu, ok)) break;
                 const uint32_t hi = sA + stage * a_bytes;
                 float2 ss[PPT];
@@ -520,7 +597,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
             // lane 0 polls the operands' barrier, the others the accumulator's
             const uint32_t bar = lane == 0 ? umma::smem_u32(&bar_af[stage]) : umma::smem_u32(&bar_te[b]);
             const uint32_t parity = lane == 0 ? (it >> a.stages_log2) & 1u : ((it / accs) & 1u) ^ 1u;
-            const bool ok = w_wait(bar, parity, abort_flag);
+            const bool ok = w_wait(bar, parity, abort_flag, a.wait_ns);
             if (!__all_sync(0xffffffffu, ok)) break;
             __syncwarp();
             umma::fence_after_sync();
@@ -566,12 +643,13 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         const float rmax = 0x1p60f * scale;
         const float2 two = make_float2(-2.0f, -2.0f);
         uint32_t b = g, phase = 0, slot = g, nx_phase = 0;  // the slots go round as the tiles of all groups do
-        for (uint32_t t = blockIdx.x + g * gridDim.x; t < a.tiles; t += EG * gridDim.x) {
+        uint32_t t = blockIdx.x + g * gridDim.x;
+        for (; t < a.tiles; t += EG * gridDim.x) {
             const uint32_t taddr = tmem + b * cols + ((q * 32u) << 16);
             const uint32_t bar_full = umma::smem_u32(&bar_tf[b]), bar_empty = umma::smem_u32(&bar_te[b]);
             // lane 0 polls the scores' barrier, the others the norms'
             const bool ok = w_wait(lane == 0 ? bar_full : umma::smem_u32(&bar_nx[slot]), lane == 0 ? phase : nx_phase,
-                                   abort_flag);
+                                   abort_flag, a.wait_ns);
             if (!__all_sync(0xffffffffu, ok)) break;
             __syncwarp();
             umma::fence_after_sync();
@@ -715,6 +793,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
                 if (a.msum) atomicAdd(&s_mass[label], 1u);
             }
         }
+        if (lane == 0) s_next[warp] = t;
     }
 
     umma::fence_before_sync();
@@ -724,10 +803,33 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         umma::fence_after_sync();
         umma::tmem_dealloc(tmem, accs * cols);
     }
+    if (s_abort) {
+        // A wait ran out and the tensor cores were given up: the CTA's other
+        // points by all clusters, a warp per 32 points, with the centroids in the
+        // operands' place if they fit.
+        T* s_c = reinterpret_cast<T*>(smem_raw + (sB - umma::smem_u32(smem_raw)));
+        const uint32_t stride = (k + 7u) & ~7u;
+        const bool rows = (size_t)d * stride * sizeof(T) <= 2u * b_part + a.stages * a_bytes;
+        if (rows)
+            for (uint32_t i = tid; i < d * k; i += W_THREADS) s_c[i / k * stride + i % k] = __ldg(a.centroids + i);
+        __syncthreads();
+        for (uint32_t w = 0; w < W_EPI_WARPS; ++w)
+            for (uint64_t t = s_next[w] + (uint64_t)warp * EG * gridDim.x; t < a.tiles;
+                 t += (uint64_t)(W_THREADS / 32) * EG * gridDim.x) {
+                const uint64_t p = t * WM + (w & 3u) * 32u;
+                if (p >= n) continue;
+                const uint32_t label = rows ? w_exact32<T, true>(a.points, n, p, s_c, stride, k, d)
+                                            : w_exact32<T, false>(a.points, n, p, a.centroids, k, k, d);
+                if (p + lane < n) {
+                    a.labels[p + lane] = (L)label;
+                    if (a.msum) atomicAdd(&s_mass[label], 1u);
+                }
+            }
+        __syncthreads();
+    }
     if (a.msum)
         for (uint32_t c = tid; c < k; c += W_THREADS)
             if (s_mass[c]) atomicAdd(&a.msum[c], (unsigned long long)s_mass[c]);
-    if (tid == 0 && s_abort && a.error) atomicExch(a.error, 1u);
 }
 
 // Dynamic shared memory of a shape: alignment, centroid halves, point stages.
@@ -763,10 +865,14 @@ int launch_wide_v(const WideArgs<T, L>& a, size_t smem, cudaStream_t s) {
 }
 
 template <typename T, typename L>
-int launch_wide_t(const T* points, const T* centroids, L* labels, unsigned long long* msum, unsigned int* error,
-                  uint64_t n, uint32_t d, uint32_t k, cudaStream_t s) {
+int launch_wide_t(const T* points, const T* centroids, L* labels, unsigned long long* msum, uint64_t n, uint32_t d,
+                  uint32_t k, cudaStream_t s) {
     const DeviceInfo& di = device_info();
-    WideArgs<T, L> a{points, centroids, labels, msum, error, n, d, k, 0, 0, 0, 0, 0, 0, 0};
+    // CKM_WIDE_TEST_WAIT_NS (tests only): the limit of the waits, which run out
+    // at 0, to check that the labels do not depend on them
+    const char* wait = std::getenv("CKM_WIDE_TEST_WAIT_NS");
+    WideArgs<T, L> a{points, centroids, labels, msum, wait ? std::strtoull(wait, nullptr, 10) : W_WAIT_NS, n, d, k,
+                     0, 0, 0, 0, 0, 0, 0};
     a.dk = (d + 15) / 16 * 16;
     a.kp = (k + 15) / 16 * 16;
     a.kblocks = (a.dk + 63) / 64;
@@ -839,12 +945,12 @@ bool wide_pays_f64(uint64_t n, uint32_t d, uint32_t k, bool fused) {
 
 int launch_wide_f32(const FusedF32& a, bool count, cudaStream_t s) {
     return launch_wide_t<float, uint32_t>(a.points, a.centroids, a.labels, count ? a.scratch.masses : nullptr,
-                                          a.scratch.ctrl ? a.scratch.ctrl + 1 : nullptr, a.n, a.d, a.k, s);
+                                          a.n, a.d, a.k, s);
 }
 
 int launch_wide_f64(const FusedF64& a, bool count, cudaStream_t s) {
     return launch_wide_t<double, uint64_t>(a.points, a.centroids, a.labels, count ? a.scratch.masses : nullptr,
-                                           a.scratch.ctrl ? a.scratch.ctrl + 1 : nullptr, a.n, a.d, a.k, s);
+                                           a.n, a.d, a.k, s);
 }
 
 }  // namespace ckm
