@@ -50,3 +50,35 @@ def test_fused_of_a_dominant_cluster(ckm, cuda, n, d, k):
     assert bool((L == 3).all()) and int(M[3]) == n and int(M.sum()) == n
     want = float(np.float32(0.1))
     assert float((N.reshape(d, k)[:, 3].double() - want).abs().max()) <= ROUND * want
+
+
+@pytest.mark.parametrize("n,d,k", [(20011, 10, 4), (20011, 128, 128), (30001, 8, 1300), (3001, 4, 6000)])
+def test_sums_beyond_the_float_range(ckm, cuda, n, d, k):
+    """Partial sums beyond FP32's range whose FP64 sums, and means, are not:
+    multiples of 2^120, with whole numbers (exact in any order) beside them, and
+    clusters with an infinite and a NaN point."""
+    import torch
+    rng = np.random.default_rng(n + k)
+    X = rng.integers(-8, 9, (n, d)).astype(np.float64)
+    X[:, ::3] = rng.integers(1, 9, X[:, ::3].shape) * 2.0 ** 120
+    lab = rng.integers(0, k, n)
+    lab[: n // 2] = 1  # long sums
+    lab[n - 1], lab[n - 2] = 2, 3
+    X[lab == 2, 1] = 5.0
+    where = np.nonzero(lab == 2)[0]
+    X[where[0], 1] = np.inf
+    X[np.nonzero(lab == 3)[0][-1], d - 1] = np.nan
+    P = np.ascontiguousarray(X.astype(np.float32).T).reshape(-1)
+    dP = torch.from_numpy(P).to(cuda)
+    dL = torch.from_numpy(lab.astype(np.int32)).to(cuda)
+    C, M, S = torch.zeros(k * d, device=cuda), torch.zeros(k, dtype=torch.int32, device=cuda), ckm.new_scratch(d, k, cuda)
+    ckm.centroid_update(dP, C, dL, M, S, n, d, k, mode=ckm.MODE_DEFER)
+    ckm.finalize(C, M, S, d, k)
+    mass = np.bincount(lab, minlength=k)
+    got = C.cpu().numpy().reshape(d, k)
+    with np.errstate(all="ignore"):
+        for f in range(d):
+            want = (np.bincount(lab, weights=X[:, f], minlength=k) / mass).astype(np.float32)
+            assert np.array_equal(got[f], want, equal_nan=True), (f, np.nonzero(got[f] != want)[0][:5])
+    assert np.isinf(got[1, 2]) and np.isnan(got[d - 1, 3])
+    assert not torch.any(S != 0)
