@@ -82,3 +82,57 @@ def test_sums_beyond_the_float_range(ckm, cuda, n, d, k):
             assert np.array_equal(got[f], want, equal_nan=True), (f, np.nonzero(got[f] != want)[0][:5])
     assert np.isinf(got[1, 2]) and np.isnan(got[d - 1, 3])
     assert not torch.any(S != 0)
+
+
+# m, q: the FP64 product of q m and the rounded reciprocal of m rounds to another
+# float than q does, q being the midpoint of two floats
+MIDPOINTS = [
+    (49, 27228575), (75, 29327761), (77, 30237505), (91, 24366061), (93, 27066901), (98, 26454107), (99, 21930277),
+    (103, 26067659), (105, 22320305), (107, 29451291), (117, 20817589), (123, 31892409), (150, 29915121),
+    (154, 30440621), (161, 27951659), (167, 32838917), (182, 31181453), (186, 27366901), (187, 32418583),
+    (191, 31270513), (196, 28632851), (197, 28231067), (198, 24992261), (206, 30796555), (210, 27534425),
+    (211, 33302149), (214, 25047515), (221, 27058693), (227, 24038417), (234, 19458689), (237, 30637779),
+    (239, 26562607), (243, 22114497), (245, 26043025), (246, 23777441), (249, 23492523), (253, 31761835),
+]
+
+
+def test_means_are_rounded_quotients(ckm, cuda):
+    """The mean is the FP64 quotient rounded to FP32, as ckm_finalize has it."""
+    import torch
+    n, d, k = 200000, 10, len(MIDPOINTS) + 1
+    X = np.zeros((n, d))
+    lab = np.full(n, k - 1)
+    at = k
+    for c, (m, q) in enumerate(MIDPOINTS):
+        # q m as two floats far apart, so that no FP32 table adds both
+        s = q * m
+        high = s >> 20 << 20
+        assert np.float32(high) == high and np.float32(s - high) == s - high
+        lab[c] = lab[n - 1 - c] = c
+        X[c, :], X[n - 1 - c, :] = high, s - high
+        lab[at:at + m - 2] = c
+        at += m - 2
+    assert at < n // 2
+    P = torch.from_numpy(np.ascontiguousarray(X.astype(np.float32).T).reshape(-1)).to(cuda)
+    mass = np.bincount(lab, minlength=k)
+    want = np.array([s / m for s, m in zip([q * m for m, q in MIDPOINTS], mass)]).astype(np.float32)
+    assert all(np.float32(np.float64(q * m) * (1.0 / m)) != w for (m, q), w in zip(MIDPOINTS, want))
+    # labels of a fused call: the centroids are far apart in a feature of its own
+    X2 = np.concatenate([X, 1000.0 * lab[:, None] * 2.0 ** 20], axis=1)
+    C = np.zeros((d + 1, k))
+    C[d] = 1000.0 * np.arange(k) * 2.0 ** 20
+    P2 = torch.from_numpy(np.ascontiguousarray(X2.astype(np.float32).T).reshape(-1)).to(cuda)
+    dC = torch.from_numpy(C.astype(np.float32).reshape(-1)).to(cuda)
+    N, L = torch.zeros((d + 1) * k, device=cuda), torch.full((n,), -1, dtype=torch.int32, device=cuda)
+    M, S = torch.zeros(k, dtype=torch.int32, device=cuda), ckm.new_scratch(d + 1, k, cuda)
+    ckm.fused(P2, dC, N, L, M, S, n, d + 1, k)
+    assert np.array_equal(L.cpu().numpy(), lab) and np.array_equal(M.cpu().numpy(), mass)
+    got = N.cpu().numpy().reshape(d + 1, k)
+    for f in range(d):
+        assert np.array_equal(got[f, : k - 1], want), (f, np.nonzero(got[f, : k - 1] != want)[0])
+    # and of a deferred centroid update with ckm_finalize
+    C1, M1, S1 = torch.zeros(d * k, device=cuda), torch.zeros_like(M), ckm.new_scratch(d, k, cuda)
+    ckm.centroid_update(P, C1, L, M1, S1, n, d, k, mode=ckm.MODE_DEFER)
+    ckm.finalize(C1, M1, S1, d, k)
+    for f in range(d):
+        assert np.array_equal(C1.cpu().numpy().reshape(d, k)[f, : k - 1], want), f
