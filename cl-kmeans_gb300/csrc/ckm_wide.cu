@@ -56,8 +56,14 @@
 // underflow: T = S + 2.02 rho (m1 + |x|^2 + S) + 2 (d + 8) 2^-149 scale^2.
 // A second-lowest score more than T above the lowest, m1, proves the label.
 // Other points take the reference's arithmetic over the clusters whose score
-// is within T of the lowest, or over all where a value is not finite or too
-// large.
+// is within T of the lowest if these are few. What is left, with more clusters in
+// reach or a value that is not finite or too large, waits until the CTA's tiles
+// are done and then takes all clusters, a warp's lanes over them; and where a
+// warp meets many unproved points (equal centroids) the CTA gives the tensor
+// cores up as after a failed wait. Labels, us, with each unproved point's clusters
+// in its own thread and now, n = 2^20 (generic or low-d kernel): every hundredth
+// point far out, d = 64, k = 256 7937, 195 (551), d = 16, k = 64 328, 51 (75); all
+// centroids equal, d = 16, k = 64 483, 144 (75); two equal 98, 83 (75).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -82,6 +88,13 @@ constexpr uint32_t W_TILE_BYTES = WM * 128u;  // one operand tile: 128 rows of 6
 constexpr uint32_t W_NX_SLOTS = 8, W_NX_ROWS = 48;
 constexpr float W_MAX_ABS = 32768.0f;         // |x| and |c| below: no fp16 overflow
 constexpr unsigned long long W_WAIT_NS = 2000000000ull;
+// What the tile loop does not resolve itself has this label until its end.
+constexpr uint32_t W_LATER = 0xffffffffu;
+constexpr uint32_t W_CANDIDATES = 4;          // fewer exact distances than this of a point in the tile loop
+// Unproved points that a warp takes before the CTA gives the tensor cores up,
+// some and a share of every tile's 32: beyond an eighth the exact labels by all
+// of the CTA's warps cost less.
+constexpr uint32_t W_UNPROVED_MIN = 16, W_UNPROVED_PER_TILE = 4;
 constexpr uint32_t W_POLL_NS = 2000;          // a poll of a barrier suspends its thread up to this long
 
 template <typename T, typename L>
@@ -315,7 +328,7 @@ __device__ __forceinline__ void w_step8(double x, const double* row, uint32_t le
 // The reference's label of point p + lane by all clusters, eight at a time; the
 // centroid of feature f and cluster c is at C[f * stride + c].  Past the last
 // point the last one is labelled.
-template <typename T, bool WORDS>
+template <typename T, bool SHARED>
 __device__ __noinline__ uint32_t w_exact32(const T* __restrict__ P, uint64_t n, uint64_t p, const T* C, uint32_t stride,
                                            uint32_t k, uint32_t d) {
     const uint64_t at = p + (threadIdx.x & 31u);
@@ -329,7 +342,7 @@ __device__ __noinline__ uint32_t w_exact32(const T* __restrict__ P, uint64_t n, 
         const T* src = first;
         const T* row = C + c0;
 #pragma unroll 4
-        for (uint32_t f = 0; f < d; ++f, src += n, row += stride) w_step8<WORDS>(__ldg(src), row, k - c0, acc);
+        for (uint32_t f = 0; f < d; ++f, src += n, row += stride) w_step8<SHARED>(__ldg(src), row, k - c0, acc);
 #pragma unroll
         for (uint32_t j = 0; j < 8; ++j)
             if (c0 + j < k && acc[j] < best) {
@@ -340,6 +353,71 @@ __device__ __noinline__ uint32_t w_exact32(const T* __restrict__ P, uint64_t n, 
     return label;
 }
 
+// The reference's label of one point by all clusters: the lanes of a warp over
+// the clusters, J per lane, U features' loads in flight.
+template <typename T, bool SHARED, uint32_t J, uint32_t U>
+__device__ __forceinline__ uint32_t w_exact1(const T* __restrict__ P, uint64_t n, uint64_t p, const T* C,
+                                             uint32_t stride, uint32_t k, uint32_t d) {
+    const uint32_t lane = threadIdx.x & 31u;
+    T best = TypeMax<T>::v();
+    uint32_t label = 0;
+    for (uint32_t c0 = lane; c0 < k + lane; c0 += 32 * J) {
+        T acc[J];
+#pragma unroll
+        for (uint32_t j = 0; j < J; ++j) acc[j] = T(0);
+        for (uint32_t f0 = 0; f0 < d; f0 += 32) {
+            const T mine = f0 + lane < d ? __ldg(P + (uint64_t)(f0 + lane) * n + p) : T(0);
+            const uint32_t left = min(32u, d - f0);
+            for (uint32_t f = 0; f < left; f += U) {
+                T c[U][J];
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+                    for (uint32_t j = 0; j < J; ++j)
+                        if (f + u < left && c0 + 32 * j < k) {
+                            const T* at = C + (size_t)(f0 + f + u) * stride + c0 + 32 * j;
+                            c[u][j] = SHARED ? *at : __ldg(at);
+                        } else {
+                            c[u][j] = T(0);
+                        }
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u) {
+                    const T x = __shfl_sync(0xffffffffu, mine, (f + u) & 31u);
+                    if (f + u < left)
+#pragma unroll
+                        for (uint32_t j = 0; j < J; ++j) {
+                            const T t = x - c[u][j];
+                            acc[j] = fma(t, t, acc[j]);
+                        }
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < J; ++j)
+            if (c0 + 32 * j < k && acc[j] < best) {
+                best = acc[j];
+                label = c0 + 32 * j;
+            }
+    }
+    // the lowest cluster of the lowest distance; none below the type's maximum: 0
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const T b = __shfl_xor_sync(0xffffffffu, best, o);
+        const uint32_t l = __shfl_xor_sync(0xffffffffu, label, o);
+        if (b < best || (b == best && l < label)) {
+            best = b;
+            label = l;
+        }
+    }
+    return label;
+}
+template <typename T, bool SHARED>
+__device__ __noinline__ uint32_t w_by_all(const T* __restrict__ P, uint64_t n, uint64_t p, const T* C, uint32_t stride,
+                                          uint32_t k, uint32_t d) {
+    if (k <= 64) return w_exact1<T, SHARED, 2, 8>(P, n, p, C, stride, k, d);
+    return w_exact1<T, SHARED, 8, 16 / sizeof(T)>(P, n, p, C, stride, k, d);
+}
+
 // EG epilogue groups, ACCS accumulators (a multiple of EG).
 template <typename T, typename L, int EG, int ACCS>
 __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const WideArgs<T, L> a) {
@@ -347,7 +425,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_af[4], bar_ae[4], bar_tf[4], bar_te[4], bar_nx[W_NX_SLOTS], bar_fin;
     __shared__ uint32_t s_tmem;
-    __shared__ unsigned int s_abort, s_cabs, s_cn_max, s_bad, s_omax;
+    __shared__ unsigned int s_abort, s_later, s_cabs, s_cn_max, s_bad, s_omax;
     __shared__ __align__(16) float s_cn[W_MAX_K];
     __shared__ __align__(16) T s_mu[W_MAX_D];     // the origin, then the shift of w_shift
     __shared__ uint32_t s_invalid[W_MAX_K / 32];
@@ -397,6 +475,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         umma::mbar_init(umma::smem_u32(&bar_fin), mma_warps);
         umma::mbar_fence_init();
         s_abort = 0u;
+        s_later = 0u;
         s_cabs = 0u;
         s_omax = 0u;
         s_cn_max = 0u;
@@ -644,6 +723,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         const float2 two = make_float2(-2.0f, -2.0f);
         uint32_t b = g, phase = 0, slot = g, nx_phase = 0;  // the slots go round as the tiles of all groups do
         uint32_t t = blockIdx.x + g * gridDim.x;
+        uint32_t allowed = W_UNPROVED_MIN;
         for (; t < a.tiles; t += EG * gridDim.x) {
             const uint32_t taddr = tmem + b * cols + ((q * 32u) << 16);
             const uint32_t bar_full = umma::smem_u32(&bar_tf[b]), bar_empty = umma::smem_u32(&bar_te[b]);
@@ -746,34 +826,48 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
             const float T_ = (S + fmaf(rho, fmaxf(m1 + nx, 0.0f) + S, t0)) * (1.0f + 0x1p-10f);
             const bool fin = m1 < INF && aa < W_MAX_ABS && cm < W_MAX_ABS && r < rmax && T_ < INF;
             const bool proved = fin && gap > T_;
-            if (__any_sync(0xffffffffu, in && !proved)) {
+            allowed += W_UNPROVED_PER_TILE;
+            const uint32_t open = __ballot_sync(0xffffffffu, in && !proved);
+            if (open) {
+                if (__popc(open) > allowed) {  // (this tile is labelled below, with the rest)
+                    *abort_flag = 1u;
+                    break;
+                }
+                allowed -= __popc(open);
                 // candidates of the unproved points, exact distances, the
                 // lexicographic (distance, index) minimum
                 const float cut = m1 + T_;
                 T best = TypeMax<T>::v();
-                uint32_t bc = 0;
+                uint32_t bc = 0, tries = in && !proved && fin ? W_CANDIDATES : 0u;
+                bool later = in && !proved && !fin;
+                if (__any_sync(0xffffffffu, tries))
 #pragma unroll 1
-                for (uint32_t cc = 0; cc < kp; cc += 16) {
-                    w_ld16(taddr + cc, v0);
-                    w_ld_wait(v0);
-                    uint32_t mask = 0;
-                    if (in && !proved) {
+                    for (uint32_t cc = 0; cc < kp; cc += 16) {
+                        w_ld16(taddr + cc, v0);
+                        w_ld_wait(v0);
+                        uint32_t mask = 0;
+                        if (tries) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (cc + i < k && (!fin || fmaf(-2.0f, v0[i], s_cn[cc + i]) <= cut)) mask |= 1u << i;
-                    }
-                    while (mask) {
-                        const uint32_t c = cc + __ffs(mask) - 1;
-                        mask &= mask - 1;
-                        const T dist = w_distance(a.points, n, p, a.centroids, k, c, d);
-                        if (dist < best) {  // ascending clusters: the lowest index wins a tie
-                            best = dist;
-                            bc = c;
+                            for (int i = 0; i < 16; ++i)
+                                if (cc + i < k && fmaf(-2.0f, v0[i], s_cn[cc + i]) <= cut) mask |= 1u << i;
                         }
+                        while (mask) {
+                            const uint32_t c = cc + __ffs(mask) - 1;
+                            mask &= mask - 1;
+                            if (--tries == 0u) {
+                                later = true;
+                                break;
+                            }
+                            const T dist = w_distance(a.points, n, p, a.centroids, k, c, d);
+                            if (dist < best) {  // ascending clusters: the lowest index wins a tie
+                                best = dist;
+                                bc = c;
+                            }
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                }
-                if (!proved) label = bc;
+                if (!proved) label = later ? W_LATER : bc;
+                if (later) s_later = 1u;
             }
             umma::fence_before_sync();
             __syncwarp();
@@ -790,7 +884,7 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
             }
             if (in) {
                 a.labels[p] = (L)label;
-                if (a.msum) atomicAdd(&s_mass[label], 1u);
+                if (a.msum && label != W_LATER) atomicAdd(&s_mass[label], 1u);
             }
         }
         if (lane == 0) s_next[warp] = t;
@@ -803,28 +897,47 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         umma::fence_after_sync();
         umma::tmem_dealloc(tmem, accs * cols);
     }
-    if (s_abort) {
-        // A wait ran out and the tensor cores were given up: the CTA's other
-        // points by all clusters, a warp per 32 points, with the centroids in the
+    if (s_abort || s_later) {
+        // The reference's labels by all clusters, with the centroids in the
         // operands' place if they fit.
+        constexpr uint32_t WARPS = W_THREADS / 32;
         T* s_c = reinterpret_cast<T*>(smem_raw + (sB - umma::smem_u32(smem_raw)));
-        const uint32_t stride = (k + 7u) & ~7u;
-        const bool rows = (size_t)d * stride * sizeof(T) <= 2u * b_part + a.stages * a_bytes;
-        if (rows)
-            for (uint32_t i = tid; i < d * k; i += W_THREADS) s_c[i / k * stride + i % k] = __ldg(a.centroids + i);
+        const uint32_t padded = (k + 7u) & ~7u;
+        const bool fits = (size_t)d * padded * sizeof(T) <= 2u * b_part + a.stages * a_bytes;
+        if (fits)
+            for (uint32_t i = tid; i < d * k; i += W_THREADS) s_c[i / k * padded + i % k] = __ldg(a.centroids + i);
         __syncthreads();
-        for (uint32_t w = 0; w < W_EPI_WARPS; ++w)
-            for (uint64_t t = s_next[w] + (uint64_t)warp * EG * gridDim.x; t < a.tiles;
-                 t += (uint64_t)(W_THREADS / 32) * EG * gridDim.x) {
-                const uint64_t p = t * WM + (w & 3u) * 32u;
-                if (p >= n) continue;
-                const uint32_t label = rows ? w_exact32<T, true>(a.points, n, p, s_c, stride, k, d)
-                                            : w_exact32<T, false>(a.points, n, p, a.centroids, k, k, d);
-                if (p + lane < n) {
-                    a.labels[p + lane] = (L)label;
-                    if (a.msum) atomicAdd(&s_mass[label], 1u);
+        const uint64_t step = (uint64_t)EG * gridDim.x;
+        // points that the tile loop left for later, one by one
+        if (s_later)
+            for (uint32_t w = 0; w < W_EPI_WARPS; ++w)
+                for (uint64_t t = blockIdx.x + (w >> 2) * (uint64_t)gridDim.x + warp * step; t < s_next[w]; t += WARPS * step) {
+                    const uint64_t p = t * WM + (w & 3u) * 32u;
+                    for (uint32_t left = __ballot_sync(0xffffffffu, p + lane < n && a.labels[p + lane] == (L)W_LATER); left;
+                         left &= left - 1u) {
+                        const uint32_t l = __ffs(left) - 1u;
+                        const uint32_t label = fits ? w_by_all<T, true>(a.points, n, p + l, s_c, padded, k, d)
+                                                    : w_by_all<T, false>(a.points, n, p + l, a.centroids, k, k, d);
+                        if (lane == l) {
+                            a.labels[p + l] = (L)label;
+                            if (a.msum) atomicAdd(&s_mass[label], 1u);
+                        }
+                    }
                 }
-            }
+        // The tensor cores were given up, because too few points were proved or
+        // because a wait ran out: the CTA's other points, a warp per 32.
+        if (s_abort)
+            for (uint32_t w = 0; w < W_EPI_WARPS; ++w)
+                for (uint64_t t = s_next[w] + warp * step; t < a.tiles; t += WARPS * step) {
+                    const uint64_t p = t * WM + (w & 3u) * 32u;
+                    if (p >= n) continue;
+                    const uint32_t label = fits ? w_exact32<T, true>(a.points, n, p, s_c, padded, k, d)
+                                                : w_exact32<T, false>(a.points, n, p, a.centroids, k, k, d);
+                    if (p + lane < n) {
+                        a.labels[p + lane] = (L)label;
+                        if (a.msum) atomicAdd(&s_mass[label], 1u);
+                    }
+                }
         __syncthreads();
     }
     if (a.msum)

@@ -1,6 +1,7 @@
-"""The tensor-core labels (ckm_wide.cu) where they are given up because a wait
-runs out: the labels are the oracle's all the same, and the counts and sums are
-theirs."""
+"""The tensor-core labels (ckm_wide.cu) where they are given up or prove little:
+waits that run out, and sets with points far outside, centroids far outside,
+equal centroids or many ties.  The labels are the oracle's either way, and the
+counts and sums are theirs."""
 import numpy as np
 import pytest
 
@@ -56,4 +57,30 @@ def test_waits_that_run_out(ckm, oracle, cuda, monkeypatch, dtype, limit_ns):
     monkeypatch.setenv("CKM_WIDE_TEST_WAIT_NS", limit_ns)
     for n, d, k in SHAPES:
         _, X, C = mixture(n, d, k)
+        check(ckm, oracle, cuda, X, C, dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("kind", ["far_points", "far_centroid", "far_centroids", "equal_centroids", "pairs", "lattice",
+                                  "few_far", "nan_points"])
+def test_sets_that_prove_little(ckm, oracle, cuda, monkeypatch, dtype, kind):
+    monkeypatch.setenv("CKM_FUSED_UMMA", "1")
+    for n, d, k in SHAPES:
+        rng, X, C = mixture(n, d, k)
+        if kind == "far_points":
+            X[::3] *= 1e5
+        elif kind == "few_far":
+            X[::100] *= 1e4
+        elif kind == "nan_points":
+            X[::50, d - 1] = np.nan
+        elif kind == "far_centroid":
+            C[k // 2] *= 1e3
+        elif kind == "far_centroids":
+            C[: k // 2] *= 10.0 ** rng.uniform(0, 6, (k // 2, 1))
+        elif kind == "equal_centroids":
+            C[:] = C[0]
+        elif kind == "pairs":
+            C[k // 2:] = C[: k - k // 2]
+        else:
+            X, C = np.round(X / 4), np.round(C / 4)
         check(ckm, oracle, cuda, X, C, dtype)
