@@ -37,23 +37,32 @@
 // minimum per two scores for the rows and one for the columns.  The index of
 // the lowest column rides in the low four bits of (column minimum - m1).
 //
-// Certificate.  With x, c the shifted and scaled operands, a >= |x|, cm >=
-// max |c|, r = a + cm, u = 2^-24, D = the features padded to 16, the scores
-// |c|^2 - 2 x.c are off by at most half of
+// Certificate.  With x, c the shifted and scaled operands, a >= |x|, r = a + |c|, u
+// = 2^-24, D = the features padded to 16, the score |c|^2 - 2 x.c of a cluster is
+// off by at most half of
 //   3.001 2^-22 r^2       the dropped x_l.c_l and the residuals of the split
 //   1.01 gamma r^2        f32 accumulation, gamma = 2 d 2^-23: two ulps per
 //                         addition; the 2 d cross products come first and
 //                         stay below 2^-10 |x||c|, so d additions count
-//   (D / 4 + 16) u r^2    |c|^2 in FP32 (5 steps and D / 8 partial sums), the
-//                         fma of the score, x and c rounded when shifted
+//   (D / 4 + 18) u r^2    |c|^2 in FP32 (5 steps, D / 8 partial sums, the factor
+//                         below), the fma of the score, x and c rounded when
+//                         shifted
 //   4.1 2^-25 sqrt(D) r   fp16's subnormal range
 //   for FP64 points, whose shift by the origin o rounds three times and whose
 //   split leaves out 2^-46 |x| (|x_f| <= |t_f| + |o_f|, t = x - o) or 2^-126:
 //   8 u r^2 and 8.2 sqrt(D) r (2^-43 max |o| + 2^-120) scale, in x.c and |c|^2
 //   2^-40                 second order
-// whose sum is S.  The reference's distance t = x - c, fma(t, t, acc) is
-// within rho = (d + 4) u of the exact one (FP32; far less in FP64), plus
-// underflow: T = S + 2.02 rho (m1 + |x|^2 + S) + 2 (d + 8) 2^-149 scale^2.
+// = t2 r^2 + t1 r + 2^-40. As r^2 <= 2 a^2 + 2 |c|^2 and |c| <= 2^-7 |c|^2 + 32, that is
+// A + w |c|^2 with A = 2 t2 a^2 + t1 a + 32 t1 + 2^-40 and w = 2 t2 + 2^-7 t1. The cluster's
+// own part is taken off its |c|^2 once (times 1 - w/2), so that the scores
+// bound the exact ones from below up to A / 2, and a far centroid widens no other
+// cluster's bound. The exact score of the lowest one's cluster c1 is at most A / 2
+// + w |c1|^2 above its own: all differences hold up to S = A + w |c1|^2. With h = m1 +
+// |x|^2, c1 is within h + S of x, squared, so |c1|^2 <= 2 a^2 + 2 (h + S) and S <= A +
+// 1.003 2 w (a^2 + h).
+// The reference's distance t = x - c, fma(t, t, acc) is within rho = (d + 4) u of the
+// exact one (FP32; far less in FP64), plus underflow: T = S + 2.02 rho (h + S)
+// + 2 (d + 8) 2^-149 scale^2.
 // A second-lowest score more than T above the lowest, m1, proves the label.
 // Other points take the reference's arithmetic over the clusters whose score
 // is within T of the lowest if these are few. What is left, with more clusters in
@@ -496,24 +505,20 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
     // ---- centroids: origin, validity, scale, fp16 halves, |c|^2 ----
     // A centroid with a coordinate that is not finite never wins in the
     // reference (its distance is not below the type's maximum): a zero row
-    // with a huge |c|^2.  The origin is the mean of the others' coordinates;
-    // any finite value would do.
+    // with a huge |c|^2.  The origin is a median of medians of 27 of the
+    // centroids, which a few far ones do not move; any finite value would do.
     for (uint32_t f = warp; f < d; f += W_THREADS / 32) {
-        T s = T(0);
-        uint32_t cnt = 0;
-        for (uint32_t c = lane; c < k; c += 32) {
-            const T v = __ldg(a.centroids + (uint64_t)f * k + c);
-            if (isfinite(v)) {
-                s += v;
-                ++cnt;
-            } else {
-                atomicOr(&s_invalid[c >> 5], 1u << (c & 31u));
-            }
+        const T* row = a.centroids + (uint64_t)f * k;
+        for (uint32_t c = lane; c < k; c += 32)
+            if (!isfinite(__ldg(row + c))) atomicOr(&s_invalid[c >> 5], 1u << (c & 31u));
+        T m = __ldg(row + (lane < 27 ? lane * k / 27 : 0u));
+#pragma unroll
+        for (uint32_t i = 0; i < 3; ++i) {  // medians of three, of 9 threes, then 3, then 1
+            const T x = __shfl_sync(0xffffffffu, m, 3 * lane), y = __shfl_sync(0xffffffffu, m, 3 * lane + 1),
+                    z = __shfl_sync(0xffffffffu, m, 3 * lane + 2);
+            m = fmax(fmin(x, y), fmin(fmax(x, y), z));
         }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        cnt = __reduce_add_sync(0xffffffffu, cnt);
-        const T mu = cnt ? s / (T)(float)cnt : T(0);
-        if (lane == 0) s_mu[f] = isfinite(mu) ? mu : T(0);
+        if (lane == 0) s_mu[f] = isfinite(m) ? m : T(0);
     }
     __syncthreads();
     {
@@ -558,10 +563,17 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         if (valid) atomicAdd(&s_cn[c], ss.x + ss.y);
     }
     __syncthreads();
+    // the certificate's constants, and |c|^2 less each cluster's part of the bound
+    const float fd = (float)d, fk = (float)dk;
+    const float t2 = (3.001f * 0x1p-22f + 1.01f * 2.0f * fd * 0x1p-23f * 1.005f + (0.25f * fk + (sizeof(T) == 4 ? 18.0f : 26.0f)) * 0x1p-24f) *
+                     1.002f;
+    const float origin = sizeof(T) == 4 ? 0.0f : fmaf(__uint_as_float(s_omax), 0x1p-43f, 0x1p-120f) * scale;
+    const float t1 = (4.1f * 0x1p-25f + 8.2f * origin) * sqrtf(fk) * 1.001f;
+    const float w = (2.0f * t2 + t1 * 0x1p-7f) * 1.001f;
     for (uint32_t c = tid; c < kp; c += W_THREADS) {
         const bool valid = c < k && !((s_invalid[c >> 5] >> (c & 31u)) & 1u) && !s_bad;
         if (valid) atomicMax(&s_cn_max, __float_as_uint(s_cn[c]));
-        else s_cn[c] = 0x1p126f;
+        s_cn[c] = valid ? s_cn[c] * (1.0f - (0.5f * w + 0x1p-24f)) : 0x1p126f;
     }
     // the padding features of the point tiles stay zero
     for (uint32_t u = warp; u < a.stages * 2 * 4; u += W_THREADS / 32)
@@ -712,11 +724,8 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
         const uint32_t g = warp >> 2, q = warp & 3u, row = q * 32 + lane;
         const float INF = __int_as_float(0x7f800000);
         const float cm = s_bad ? INF : sqrtf(__uint_as_float(s_cn_max)) * (1.0f + 0x1p-16f);
-        const float fd = (float)d, fk = (float)dk;
-        const float t2 = (3.001f * 0x1p-22f + 1.01f * 2.0f * fd * 0x1p-23f * 1.005f + (0.25f * fk + (sizeof(T) == 4 ? 16.0f : 24.0f)) * 0x1p-24f) *
-                         1.002f;
-        const float origin = sizeof(T) == 4 ? 0.0f : fmaf(__uint_as_float(s_omax), 0x1p-43f, 0x1p-120f) * scale;
-        const float t1 = (4.1f * 0x1p-25f + 8.2f * origin) * sqrtf(fk) * 1.001f;
+        const float t00 = t1 * 32.0f + 0x1p-40f, wc = 2.0f * (w * 1.001f + 0x1p-22f) * 1.003f;
+        const float ta = 2.0f * t2 + wc;
         const float rho = sizeof(T) == 4 ? 2.02f * (fd + 4.0f) * 0x1p-24f * 1.001f : 0x1p-40f;
         const float t0 = 2.0f * (fd + 8.0f) * 0x1p-149f * scale * scale;
         const float rmax = 0x1p60f * scale;
@@ -821,10 +830,10 @@ __global__ void __launch_bounds__(w_threads(EG), 1) wide_label_kernel(const Wide
             for (uint32_t i = 0; i < nx_parts; ++i) nx += s_nx[slot * nx_parts + i][row];
             nx *= 1.0f + 0x1p-15f;
             const float aa = sqrtf(nx) * (1.0f + 0x1p-16f);
-            const float r = (aa + cm) * (1.0f + 0x1p-20f);
-            const float S = fmaf(t2 * r, r, fmaf(t1, r, 0x1p-40f));
-            const float T_ = (S + fmaf(rho, fmaxf(m1 + nx, 0.0f) + S, t0)) * (1.0f + 0x1p-10f);
-            const bool fin = m1 < INF && aa < W_MAX_ABS && cm < W_MAX_ABS && r < rmax && T_ < INF;
+            const float h = fmaxf(m1 + nx, 0.0f);
+            const float S = fmaf(ta * aa, aa, fmaf(t1, aa, fmaf(wc, h, t00)));
+            const float T_ = (S + fmaf(rho, h + S, t0)) * (1.0f + 0x1p-10f);
+            const bool fin = m1 < INF && aa < W_MAX_ABS && cm < W_MAX_ABS && aa + cm < rmax && T_ < INF;
             const bool proved = fin && gap > T_;
             allowed += W_UNPROVED_PER_TILE;
             const uint32_t open = __ballot_sync(0xffffffffu, in && !proved);
