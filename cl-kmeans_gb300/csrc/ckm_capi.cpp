@@ -106,7 +106,7 @@ int dispatch_fused_f32(const FusedF32& a, cudaStream_t s) {
 int dispatch_fused_f64(const FusedF64& a, cudaStream_t s) {
     const char* e = getenv("CKM_FUSED_UMMA");
     const bool forced = e && e[0] == '1' && wide_supported(a.n, a.d, a.k);
-    if (!forced && lowd64_pays(a.n, a.d, a.k) && sums_pays_f64(a.n, a.d, a.k)) {
+    if (!forced && lowd64_pays(a.n, a.d, a.k) && sums_supported_f64(a.n, a.d, a.k)) {
         const int st = launch_lowd64(a, true, s);
         return st ? st : launch_sums_f64(a, false, s);
     }

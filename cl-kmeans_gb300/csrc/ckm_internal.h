@@ -111,6 +111,7 @@ bool rows_supported(uint32_t d, uint32_t k);  // the fixed-d kernel of ckm_gener
 // sums_pays: where a centroid update takes it.
 bool sums_pays_f32(uint64_t n, uint32_t d, uint32_t k);
 bool sums_pays_f64(uint64_t n, uint32_t d, uint32_t k);
+bool sums_supported_f64(uint64_t n, uint32_t d, uint32_t k);  // (FP32: wherever wide_supported)
 uint64_t sums_partials_f32(uint64_t n, uint32_t d, uint32_t k);
 int launch_sums_f32(const FusedF32& a, bool count, uint64_t partials, cudaStream_t s);
 int launch_sums_f64(const FusedF64& a, bool count, cudaStream_t s);
