@@ -126,7 +126,9 @@ int dispatch_labeling_f32(const FusedF32& a, cudaStream_t s) {
 }
 
 int dispatch_labeling_f64(const FusedF64& a, cudaStream_t s) {
-    if (lowd64_pays(a.n, a.d, a.k)) return launch_lowd64(a, false, s);
+    // (two clusters on few points: n = 20000 d = 8 5.2 us, the generic kernel 4.8)
+    const bool tiny = a.k <= 2 && a.d >= 8 && a.n < 65536;
+    if (!tiny && lowd64_pays(a.n, a.d, a.k)) return launch_lowd64(a, false, s);
     if (wide_pays_f64(a.n, a.d, a.k, false) && wide_supported(a.n, a.d, a.k)) return launch_wide_f64(a, false, s);
     return launch_generic_f64(a, Pass::LabelOnly, s);
 }

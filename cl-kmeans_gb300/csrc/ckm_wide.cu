@@ -1028,9 +1028,10 @@ bool wide_supported(uint64_t n, uint32_t d, uint32_t k) {
 // sums pass). A tile of this kernel costs most of its time whatever k and d
 // are, so it wins where k*d is large, and labels alone also want enough tiles
 // to pay for its set-up of 3 to 4 us.
-//   low-d kernel (fused):    n = 5000 d = 8 k = 64 27 / 19, n = 2e5 34 / 29, n = 4e6 190 /
-//                            172; n = 1.1e6 d = 16 k = 40 84 / 75, d = 12 k = 45 73 / 82
-//                (labels):   d = 8 k = 64 n = 5e4 7.1 / 10.5, n = 10^6 38 / 35;
+//   low-d kernel (fused):    n = 5000 d = 8 k = 64 27 / 19, n = 10^5 level, n = 2^20 64 /
+//                            72, k = 80 level, k = 100 1.45 times the speed; n =
+//                            1.1e6 d = 16 k = 40 84 / 75, d = 12 k = 45 73 / 82
+//                (labels):   d = 8 k = 64 n = 5e4 7.1 / 10.5, n = 10^6 38 / 37;
 //                            d = 16 k = 32 n = 5e4 5.0 / 6.7, n = 5e5 21 / 19;
 //                            d = 16 k = 64 n = 5000 7.5 / 6.6, d = 8 k = 128 n =
 //                            5e4 12 / 15; at n = 2^20 d = 16 k = 16 25 / 33, d = 4
@@ -1040,18 +1041,26 @@ bool wide_supported(uint64_t n, uint32_t d, uint32_t k) {
 //               (labels):    d = 32 k = 20 n = 10^5 9.5 / 11, d = 64 k = 10 n = 3e5
 //                            21 / 23; d = 32 k = 64 n = 5000 5.8 / 8.2, n = 20000
 //                            8.5 / 8.3, n = 3e5 38 / 19
-//   generic kernel (fused):  n = 5000 d = 10 k = 4 18 / 14, d = 40 k = 3 47 / 15
+//   generic kernel (fused):  n = 5000 d = 10 k = 4 18 / 14, d = 40 k = 3 47 / 15; d = 10 n
+//                            = 20000 0.75 to 0.9 times the speed for k = 8 to 24, 1.1
+//                            for k = 32; n = 10^5 0.9 for k = 8 to 16, n = 4e5 above 1
+//                            (its shared atomics meet most in two or three rows)
 //               (labels):    d = 20 k = 20 n = 5000 10.3 / 7.1, d = 33 k = 10 8.2 /
 //                            7.0; d = 20 k = 10 n = 5000 6.0 / 7.1, n = 3e5 23 / 17;
-//                            at n = 2^20 d = 17 k = 8 49 / 47, d = 28 k = 4 43 / 52
+//                            at n = 2^20 d = 17 k = 8 49 / 47, d = 28 k = 4 43 / 52, d
+//                            = 33 k = 5 58 / 65, d = 48 k = 5 81 / 63, k = 3 56 / 63; d = 80
+//                            k = 5 n = 10^5 0.9, n = 4e5 1.3, k = 2 n = 4e5 0.7
 bool wide_pays_f32(uint64_t n, uint32_t d, uint32_t k, bool fused) {
     const uint64_t kd = (uint64_t)k * d;
     if (lowd_supported(d, k)) {
-        const uint64_t from = d == 12 ? 640 : 512;  // (a second chunk of four features costs like one of eight)
+        // (a second chunk of four features costs like one of eight)
+        const uint64_t from = d == 12 || (d == 8 && n >= 65536) ? 640 : 512;
         return (fused || n >= (1u << 19)) ? d >= 8 && kd >= from : d >= 12 && kd >= 1024;
     }
     if ((d == 32 || d == 64) && rows_supported(d, k)) return fused ? kd >= 640 : kd >= 1024 && n >= 16384;
-    return fused || kd >= 320 || (kd >= 136 && n * kd >= (1u << 25));
+    if (fused) return d >= 16 || k <= 4 || kd >= 300 || n >= (1u << 18);
+    if (k >= 8) return kd >= 330 || (kd >= 136 && n * kd >= (1u << 25));
+    return k >= 4 && (kd >= 480 || (kd >= 176 && n * kd >= (1u << 26)));
 }
 // FP64 (the generic kernel against this one; d <= 16 mostly goes to
 // ckm_lowd64.cu): its FP64 distances grow with k*d, so few of them want many points.
