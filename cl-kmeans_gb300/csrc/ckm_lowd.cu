@@ -38,14 +38,19 @@ constexpr int BLK = 256;
 // (n = 2^20, d = 4, k = 10: 19.9 us without, 14.2 with; labels alone 8.1).  Not
 // with few tiles (n = 10^5, d = 8, k = 16, 98 tiles: 13.0 without, 14.1 with),
 // nor with few sums (n = 1.1e6, d = 4, k = 2: 9.1 without, 10.5 with), nor with
-// four or more tiles per resident CTA, where the SMs that whole clusters leave
-// idle cost more (n = 2e6, d = 4, k = 16: 24.5 without, 22.6 with; n = 1.5e6, d =
-// 6, k = 61, 4.8 tiles: 66.6 without, 70.2 with).  The sums alone are merged CTA
-// by CTA (n = 1.2e6, d = 2, k = 43: 12.8, 15.3 with clusters).
+// four or more tiles per resident CTA (with many clusters to compare with, two),
+// where the SMs that whole clusters leave idle cost more (n = 2e6, d = 4, k = 16:
+// 24.5 without, 22.6 with; n = 1.5e6, d = 6, k = 61, 4.8 tiles: 66.6 without, 70.2
+// with; n = 2^20, d = 8, 3.4 tiles, 0.90 to 0.94 times the speed from k = 32 on, 1.04
+// and more below; d = 4, k = 180, one CTA per SM, 3.4 tiles, 0.86, k = 128, two, 1.02).
+// The sums alone are merged CTA by CTA (n = 1.2e6, d = 2, k = 43: 12.8, 15.3 with
+// clusters), and so are spatially ordered points, whose CTAs have sums of few
+// clusters each (n = 2e5, d = 8, k = 16 12.6, 14.5 with clusters; n = 2^19, d = 4, k =
+// 32 15.0, 16.8).
 constexpr uint32_t LOWD_CLUSTER = 8;
 constexpr uint64_t LOWD_CLUSTER_MIN_TILES = 128;
-constexpr uint64_t LOWD_CLUSTER_MAX_PER_CTA = 4;
-constexpr uint32_t LOWD_CLUSTER_MIN_SUMS = 32;  // k (d + 1)
+constexpr uint64_t LOWD_CLUSTER_MAX_PER_CTA = 4, LOWD_CLUSTER_MAX_MANY = 2;
+constexpr uint32_t LOWD_CLUSTER_MIN_SUMS = 32, LOWD_CLUSTER_MANY_SUMS = 240;  // k (d + 1)
 
 template <int D> struct LowdCfg {
     static constexpr int PPT = D <= 4 ? 8 : (D <= 8 ? 4 : 2);  // points per thread per tile
@@ -524,6 +529,8 @@ int launch_lowd_c(const FusedF32& a, cudaStream_t s) {
     const uintptr_t la = reinterpret_cast<uintptr_t>(a.labels);
     const int vec_ok = (a.n % VW == 0) && (pa % (VW * 4) == 0) && (la % (VW * 4) == 0);
     if constexpr (CLUSTER) {
+        const uint64_t most = a.k * (D + 1) > LOWD_CLUSTER_MANY_SUMS ? LOWD_CLUSTER_MAX_MANY : LOWD_CLUSTER_MAX_PER_CTA;
+        if (ntiles >= most * grid) return launch_lowd_c<D, PPT, ACC, PASS, NT, MINB, PREF, PRUNE, false>(a, s);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -568,11 +575,9 @@ int launch_lowd_c(const FusedF32& a, cudaStream_t s) {
 
 template <int D, int PPT, int ACC, Pass PASS, int NT, int MINB, bool PREF, bool PRUNE = false>
 int launch_lowd_v(const FusedF32& a, cudaStream_t s) {
-    if constexpr (PASS == Pass::Fused) {
+    if constexpr (PASS == Pass::Fused && !PRUNE) {
         const uint64_t ntiles = (a.n + (uint64_t)NT * PPT - 1) / ((uint64_t)NT * PPT);
-        const uint64_t per_cta = ntiles / ((uint64_t)device_info().sm_count * MINB);
-        if (ntiles >= LOWD_CLUSTER_MIN_TILES && per_cta < LOWD_CLUSTER_MAX_PER_CTA &&
-            a.k * (D + 1) >= LOWD_CLUSTER_MIN_SUMS)
+        if (ntiles >= LOWD_CLUSTER_MIN_TILES && a.k * (D + 1) >= LOWD_CLUSTER_MIN_SUMS)
             return launch_lowd_c<D, PPT, ACC, PASS, NT, MINB, PREF, PRUNE, true>(a, s);
     }
     return launch_lowd_c<D, PPT, ACC, PASS, NT, MINB, PREF, PRUNE, false>(a, s);
