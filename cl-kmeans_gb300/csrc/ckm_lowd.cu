@@ -17,7 +17,7 @@
 //     (fused_feature_sum.hpp:224-439);
 //   - the last CTA to finish divides sums by masses
 //     (MatrixBinaryOp::row divide, matrix_binary_op.cl:98-114) and re-zeroes
-//     the scratch, so a whole Lloyd iteration is one launch.
+//     the scratch, so a Lloyd iteration on this kernel is one launch.
 #include "ckm_device.cuh"
 #include "ckm_internal.h"
 

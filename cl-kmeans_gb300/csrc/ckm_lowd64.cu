@@ -26,9 +26,10 @@
 // an infinite or NaN coordinate, or one beyond the float range, makes them not
 // so.  A centroid that is not finite is never the nearest: its score is +inf.
 //
-// What bounds it: the FP32 pipe, 4 d k packed operations per two points and
-// some 5 k for the lowest two.  n = 2^20, d = 4, k = 16 18 us, with the 42 MB
-// read and written 7 (the tensor-core labels 51, the generic kernel 278).
+// What bounds it: issue slots (66 % at d = 4, k = 16), of which the lowest two and
+// the integer split take the ALU pipe to 52 %, the 4 d k packed operations per two
+// points the FMA pipe to 29 %.  n = 2^20, d = 4, k = 16 18 us, with the 42 MB read
+// and written 7 (the tensor-core labels 51, the generic kernel 278).
 #include "ckm_device.cuh"
 #include "ckm_internal.h"
 

@@ -1018,6 +1018,9 @@ int launch_wide_t(const T* points, const T* centroids, L* labels, unsigned long 
 
 }  // namespace
 
+// The ends in d and k are those of the kernel's shared and tensor memory: at d =
+// 129 or k = 257 the generic kernel takes over, some ten times slower. Nothing in
+// the kernel needs the end in n; larger sets have not been run here.
 bool wide_supported(uint64_t n, uint32_t d, uint32_t k) {
     const DeviceInfo& di = device_info();
     if (di.cc_major != 10 || n == 0 || n >= ((uint64_t)1 << 29) || d > W_MAX_D || k < 2 || k > W_MAX_K) return false;

@@ -153,7 +153,7 @@ public:
                       datapoint, events);
     }
 
-    // Any mode (FINALIZE = one whole Lloyd iteration in one launch).
+    // Any mode (FINALIZE = one whole Lloyd iteration in one call).
     Event launch(const Stream& queue, size_t d, size_t n, size_t k, const PointT* points, const PointT* old_c,
                  PointT* new_c, LabelT* labels, MassT* masses, int mode, Measurement::DataPoint& dp,
                  WaitList const& events) {

@@ -101,12 +101,16 @@ int ckm_scratch_init(void *scratch, size_t scratch_bytes, ckm_stream_t stream);
 /* and FusedClusterMerge::operator() (cl_kernels/fused_cluster_merge.hpp:   */
 /* 193-414).  The kernel is picked by shape: labels on the tensor cores     */
 /* (tcgen05) and a pass of feature sums for d <= 128 and 2 <= k <= 256      */
-/* where that is faster (FP32: d >= 8 with k*d >= 512, every d without a    */
-/* kernel of its own); for FP64 and d <= 16 an FP32-screened labeling before */
-/* the sums unless k*d is large; else one launch of the low-d               */
-/* kernel (d = 1-8, 12, 16), the rows kernel (d = 32, 64) or the generic    */
-/* kernel.  Scratch holds 4 KiB more than they use for d = 32 / 64 with     */
-/* 16 <= k <= 256.  The labels are the reference's on every path.           */
+/* where that is faster (FP32: d >= 8 with k*d from 512 or 640 on, most     */
+/* shapes without a kernel of their own); for FP64 and d <= 16 an           */
+/* FP32-screened labeling before the sums unless k*d is large; else one     */
+/* launch of the low-d kernel (d = 1-8, 12, 16), the rows kernel (d = 32,   */
+/* 64) or the generic kernel.  Scratch holds 4 KiB more than they use for   */
+/* d = 32 / 64 with 16 <= k <= 256.  The labels are the reference's on      */
+/* every path.                                                              */
+/* labels is written and may be read again before the call has completed    */
+/* on its stream: nothing else, another call with the same buffer           */
+/* included, may write it until then.                                       */
 /* ---------------------------------------------------------------------- */
 int ckm_fused_f32(uint32_t num_features, uint64_t num_points, uint32_t num_clusters,
                   const float *points, const float *old_centroids, float *new_centroids,
