@@ -104,7 +104,11 @@ constexpr uint32_t W_CANDIDATES = 4;          // fewer exact distances than this
 // some and a share of every tile's 32: beyond an eighth the exact labels by all
 // of the CTA's warps cost less.
 constexpr uint32_t W_UNPROVED_MIN = 16, W_UNPROVED_PER_TILE = 4;
-constexpr uint32_t W_POLL_NS = 2000;          // a poll of a barrier suspends its thread up to this long
+// A poll of a barrier suspends its thread up to this long: labels of n = 2^20, d =
+// 64, k = 256 142 us with 2 us (polls that run out within a tile), 141 with 6, 140.3
+// with 20; a CTA that gives up leaves that much later (all centroids equal, d = 16,
+// k = 64: 144, 144 and 162 us).
+constexpr uint32_t W_POLL_NS = 6000;
 
 template <typename T, typename L>
 struct WideArgs {
